@@ -28,7 +28,7 @@ P, I64, I32, U64 = C.c_void_p, C.c_int64, C.c_int32, C.c_uint64
 def build(reference: bool = True) -> None:
     """Builds liboracle.so and, when the reference sources are present, _ref."""
     subprocess.run(["make", "-s", "-C", str(HERE), "oracle"], check=True)
-    if reference and REFERENCE_SRC.exists():
+    if reference and (REFERENCE_SRC / "src").is_dir():
         jobs = str(min(16, os.cpu_count() or 4))
         subprocess.run(["make", "-s", "-C", str(HERE), f"-j{jobs}", "ref", f"REF={REFERENCE_SRC}"], check=True)
         # the drop-in driver links the product library, built before this step
