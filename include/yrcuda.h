@@ -351,25 +351,19 @@ yrc_status yrc_accel_autotune(yrc_accel* accel, const yrc_ray* rays, int64_t cou
                               float* times_ms);
 /* Set / get the launch shape (0..YRC_TRACE_SHAPES-1) used for closest-hit
  * (any_hit = 0) or any-hit (any_hit = 1) traces; 0 is the default shape.
- * Shapes 0-6 differ in block size, node visits between ray refills and
- * register budget; shapes 7, 8 and 9 let a lane that reaches a leaf wait
- * until 4, 8 or 16 lanes of its warp are at leaves (or none is at an
- * interior node), so that the leaf tests run for many lanes at once;
- * shapes 10 and 11 are shape 8 with a 40-register budget (12 blocks of 128
- * per SM) and with blocks of 256, shape 12 is shape 9 with a 64-register
- * budget (8 blocks of 128 per SM; the two-level kernel needs more), and
- * shapes 13 and 14 are shape 8 refilling lanes every 16 and 32 steps
- * (every 2 and 4 steps measured slower), shapes 15 and 16 shape 8 with
- * register budgets for 9 and 10 blocks of 128 per SM. No
- * shape changes a hit: every ray keeps the reference's visiting order. */
+ * Every shape lets a lane that reaches a leaf wait until several lanes of its
+ * warp are at leaves (or none is at an interior node), so that the leaf
+ * tests run for many lanes at once: shapes 9 and 12 until 16 lanes are, the
+ * others until 8 (shapes 10, 15 and 16 with a register budget for 9 blocks of
+ * 128 per SM). Over quantised nodes (flat BVHs of triangles only from 256
+ * interior nodes on, and two-level BVHs of such) the kernels have budgets and
+ * batches of their own. No shape changes a hit. */
 yrc_status yrc_accel_set_trace_shape(yrc_accel* accel, int32_t any_hit, int32_t shape);
 int32_t yrc_accel_get_trace_shape(const yrc_accel* accel, int32_t any_hit);
 
 /* The launch shape of yrc_trace_host's traversal kernels: its chunks'
  * kernels run beside the chunks' host<->device copies, and the shape that
- * is fastest alone is not always the fastest there (on the 2M-triangle
- * set the leaf-batched shape 8 traverses 1.31x faster alone but the host
- * pipeline runs 8 % slower with it than with shape 10). autotune_host
+ * is fastest alone is not always the fastest there. autotune_host
  * times yrc_trace_host on `count` HOST rays (pinned memory, as the caller's
  * own) once per shape and keeps the lowest-numbered shape within 2 % of the
  * fastest; set_host_trace_shape(-1) makes the host path follow

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "device_layout.cuh"
+#include "quantise.hpp"
 #include "trace_kernels.hpp"
 #include "yrc_internal.hpp"
 
@@ -25,6 +26,10 @@ struct Layout {
     std::vector<NodePair> pairs;
     std::vector<Record> records;
     std::vector<Instance> instances;
+    // The BVHs in the order of their pairs, for the quantised copy; empty
+    // where the BVH may not have one.
+    std::vector<QRange> ranges;
+    int32_t quantised_stack = 0;  // deepest stack its traversal may need
 };
 
 Record SkipRecord(int32_t kind) {
@@ -51,6 +56,7 @@ bool AddBvh(const yrc_bvh_node* nodes, int64_t node_count, SlotFn slot_record, L
     const size_t n = static_cast<size_t>(node_count);
     std::vector<int32_t> ref(n, kUnassigned);
     std::vector<int32_t> sub_depth(n, 0);
+    std::vector<int32_t> sub_first(n, 0);  // first record of the subtree
     std::vector<uint8_t> color(n, 0);  // 0 white, 1 on the DFS path, 2 done
     struct Frame {
         int32_t node;
@@ -81,6 +87,7 @@ bool AddBvh(const yrc_bvh_node* nodes, int64_t node_count, SlotFn slot_record, L
                 Record& last = out.records.back();
                 last.v1.w = IntBits(FloatBits(last.v1.w) | kRecLast);
                 ref[i] = ~first;
+                sub_first[i] = first;
                 color[i] = 2;
                 stack.pop_back();
                 continue;
@@ -110,7 +117,9 @@ bool AddBvh(const yrc_bvh_node* nodes, int64_t node_count, SlotFn slot_record, L
         p.a = make_float4(lb[0], lb[1], lb[2], lb[3]);
         p.b = make_float4(lb[4], lb[5], rb[0], rb[1]);
         p.c = make_float4(rb[2], rb[3], rb[4], rb[5]);
-        p.d = make_int4(l >= 0 ? ref[l] : kAbsentRef, r >= 0 ? ref[r] : kAbsentRef, 0, 0);
+        sub_first[i] = l >= 0 ? sub_first[l] : (r >= 0 ? sub_first[r] : 0);
+        p.d = make_int4(l >= 0 ? ref[l] : kAbsentRef, r >= 0 ? ref[r] : kAbsentRef,
+                        l < 0 ? INT32_MIN : (r < 0 ? INT32_MAX : sub_first[r]), 0);
         int32_t d = 0;
         if (l >= 0) d = std::max(d, sub_depth[l]);
         if (r >= 0) d = std::max(d, sub_depth[r]);
@@ -315,13 +324,15 @@ struct yrc_accel {
     int device = 0;
     int sm_count = 148;
     yrc::NodePair* d_pairs = nullptr;
+    yrc::QNode* d_qnodes = nullptr;      // quantised copy, nullptr where the exact nodes are traversed
+    float4* d_leaf_boxes = nullptr;      // exact leaf boxes, in the allocation of d_qnodes
     yrc::WideNode* d_wide = nullptr;  // four-wide copy, built on the first yrc_accel_set_wide(1)
     bool wide_enabled = false;
     bool triangles_only = false;  // flat BVH without spheres: a four-wide copy is allowed
     int64_t pair_count = 0;
     yrc::Record* d_records = nullptr;
     yrc::Instance* d_instances = nullptr;
-    unsigned long long* d_counter = nullptr;
+    unsigned long long* d_counter = nullptr;  // work counter, then the undecided rays (TraceArgs)
     int* d_error = nullptr;
     yrc::AccelParams params{};
     int trace_shape[2] = {0, 0};  // launch shape for closest / any hit (autotuned)
@@ -369,6 +380,7 @@ void FreeAccel(yrc_accel* a) {
     if (!a) return;
     cudaSetDevice(a->device);
     cudaFree(a->d_pairs);
+    cudaFree(a->d_qnodes);
     cudaFree(a->d_wide);
     cudaFree(a->d_records);
     cudaFree(a->d_instances);
@@ -430,15 +442,27 @@ yrc_status Finalize(Layout& layout, int32_t root_ref, const float lo[3], const f
     }
     auto* a = new (std::nothrow) yrc_accel();
     if (!a) return Fail(YRC_ERR_OUT_OF_MEMORY, "host allocation failed");
+    const int32_t absent = ~static_cast<int32_t>(layout.records.size());
+    layout.records.push_back(SkipRecord(kRecSkip));
+    layout.records.back().v1.w = IntBits(kRecSkip << 1 | kRecLast);
     cudaError_t err = cudaGetDevice(&a->device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&a->sm_count, cudaDevAttrMultiProcessorCount, a->device);
     if (err == cudaSuccess) err = Upload(&a->d_pairs, layout.pairs, a->device_bytes);
     if (err == cudaSuccess) err = Upload(&a->d_records, layout.records, a->device_bytes);
     a->pair_count = static_cast<int64_t>(layout.pairs.size());
     if (err == cudaSuccess) err = Upload(&a->d_instances, layout.instances, a->device_bytes);
-    if (err == cudaSuccess) err = cudaMalloc(reinterpret_cast<void**>(&a->d_counter), sizeof(unsigned long long));
+    if (err == cudaSuccess) err = cudaMalloc(reinterpret_cast<void**>(&a->d_counter), sizeof(unsigned long long) * (1 + kUndecidedWords));
     if (err == cudaSuccess) err = cudaMalloc(reinterpret_cast<void**>(&a->d_error), sizeof(int));
     if (err == cudaSuccess) err = cudaMemset(a->d_error, 0, sizeof(int));
+    // Small trees keep the exact nodes: they sit in L1, and a ray's few steps do
+    // not pay for setting it up against the grid (a Cornell box of 36
+    // triangles, 256 x 256 x 64 samples: 7.03 ms against 7.44 quantised).
+    bool quantised = false;
+    if (err == cudaSuccess && !layout.ranges.empty() && layout.quantised_stack <= kQuantisedStack &&
+        depth + 1 <= kQuantisedExactStack && a->pair_count >= kQuantisedMinPairs) {
+        err = Quantise(a->d_pairs, a->pair_count, static_cast<int64_t>(layout.records.size()), absent, layout.ranges,
+                       &a->d_qnodes, &a->d_leaf_boxes, &a->device_bytes, &quantised);
+    }
     if (err != cudaSuccess) {
         FreeAccel(a);
         return CudaFail(err, "accelerator upload");
@@ -457,6 +481,13 @@ yrc_status Finalize(Layout& layout, int32_t root_ref, const float lo[3], const f
     p.wide = nullptr;
     p.wide_root = kAbsentRef;
     p.wide_stack_limit = 0;
+    p.qnodes = a->d_qnodes;
+    p.leaf_boxes = a->d_leaf_boxes;
+    if (quantised) {
+        const QRange& top = layout.ranges.back();  // the flat BVH, or the TLAS behind its BLASes
+        for (int k = 0; k < 3; ++k) p.qlo[k] = top.lo[k];
+        p.qcell = top.cell;
+    }
     *out = a;
     return Ok();
 }
@@ -484,6 +515,7 @@ yrc_status LaunchInternal(yrc_accel* a, const yrc_ray* rays, int64_t count, int3
     args.triangle_tests = tt;
     args.sphere_tests = st;
     args.counter = counter;
+    args.undecided = counter + 1;
     args.error = a->d_error;
     const bool any = (flags & YRC_TRACE_ANY) != 0;
     const bool stats = (flags & YRC_TRACE_STATS) != 0;
@@ -502,7 +534,7 @@ yrc_status LaunchInternal(yrc_accel* a, const yrc_ray* rays, int64_t count, int3
         args.order = a->order.order;
     }
     if (timed && err == cudaSuccess) err = cudaEventRecord(a->ev[1], stream);
-    if (err == cudaSuccess) err = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
+    if (err == cudaSuccess) err = cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), stream);
     if (err != cudaSuccess) return CudaFail(err, "trace counter reset");
     err = LaunchTrace(args, any, stats, shape >= 0 ? shape : a->trace_shape[any ? 1 : 0], stream, a->sm_count);
     if (err != cudaSuccess) return CudaFail(err, "trace launch");
@@ -604,6 +636,8 @@ yrc_status yrc_accel_create_flat(const yrc_geometry* geometry, const yrc_bvh_vie
     int32_t root = kAbsentRef, depth = 0;
     float lo[3], hi[3];
     try {
+        layout.pairs.reserve(static_cast<size_t>(bvh->node_count / 2 + 1));
+        layout.records.reserve(static_cast<size_t>(bvh->primitive_index_count) + 1);
         auto slot = [&](int64_t s) { return TriangleOrSphereRecord(*geometry, *bvh, s); };
         if (!AddBvh(bvh->nodes, bvh->node_count, slot, layout, root, lo, hi, depth, error)) {
             return Fail(YRC_ERR_INVALID_ARGUMENT, "yrc_accel_create_flat: " + error);
@@ -611,14 +645,19 @@ yrc_status yrc_accel_create_flat(const yrc_geometry* geometry, const yrc_bvh_vie
     } catch (const std::bad_alloc&) {
         return Fail(YRC_ERR_OUT_OF_MEMORY, "yrc_accel_create_flat: host allocation failed");
     }
+    // A four-wide or quantised copy is allowed for triangle-only BVHs: their
+    // closest hit does not depend on the visiting order (ties go to the
+    // smaller flat index), while a sphere tie goes to the first visited.
+    bool triangles_only = true;
+    for (int64_t i = 0; i < bvh->primitive_count; ++i) triangles_only = triangles_only && bvh->primitives[i].kind == 0;
+    if (triangles_only && root != kAbsentRef) {
+        QRange r{};
+        if (MakeQRange(0, root, lo, hi, r)) layout.ranges.push_back(r);
+        layout.quantised_stack = QuantisedStack(depth);
+    }
     const yrc_status st = Finalize(layout, root, lo, hi, 0, depth, out);
     if (st != YRC_OK) return st;
     ResolveNoAllocScratch(*out);
-    // A four-wide copy is allowed for triangle-only BVHs: their closest hit
-    // does not depend on the visiting order (ties go to the smaller flat
-    // index), while a sphere tie goes to the first visited.
-    bool triangles_only = true;
-    for (int64_t i = 0; i < bvh->primitive_count; ++i) triangles_only = triangles_only && bvh->primitives[i].kind == 0;
     (*out)->triangles_only = triangles_only;
     return st;
 }
@@ -642,18 +681,33 @@ yrc_status yrc_accel_create_two_level(const yrc_geometry* geometry, const yrc_tw
         // BLASes first so their refs are known when instances are written.
         std::vector<int32_t> blas_root(static_cast<size_t>(tl->blas_count), kAbsentRef);
         std::vector<std::array<float, 6>> blas_box(static_cast<size_t>(tl->blas_count));
+        std::vector<QRange> ranges(static_cast<size_t>(tl->blas_count));
+        bool quantise = true;  // no spheres anywhere, a grid for every BLAS
         int32_t blas_depth = 0;
+        int64_t node_total = std::max<int64_t>(tl->tlas_node_count, 0);
+        int64_t slot_total = std::max<int64_t>(tl->tlas_primitive_index_count, 0);
+        for (int32_t b = 0; b < tl->blas_count; ++b) {
+            node_total += std::max<int64_t>(tl->blases[b].bvh.node_count, 0);
+            slot_total += std::max<int64_t>(tl->blases[b].bvh.primitive_index_count, 0);
+        }
+        layout.pairs.reserve(static_cast<size_t>(node_total / 2 + 1));
+        layout.records.reserve(static_cast<size_t>(slot_total) + 1);
         for (int32_t b = 0; b < tl->blas_count; ++b) {
             const yrc_bvh_view& v = tl->blases[b].bvh;
             if (!CheckBvh(&v, error)) return Fail(YRC_ERR_INVALID_ARGUMENT, "BLAS " + std::to_string(b) + ": " + error);
             auto slot = [&](int64_t s) { return TriangleOrSphereRecord(*geometry, v, s); };
             float blo[3], bhi[3];
             int32_t d = 0;
+            const int64_t begin = static_cast<int64_t>(layout.pairs.size());
             if (!AddBvh(v.nodes, v.node_count, slot, layout, blas_root[b], blo, bhi, d, error)) {
                 return Fail(YRC_ERR_INVALID_ARGUMENT, "BLAS " + std::to_string(b) + ": " + error);
             }
             blas_depth = std::max(blas_depth, d);
             blas_box[b] = {blo[0], blo[1], blo[2], bhi[0], bhi[1], bhi[2]};
+            ranges[b].begin = begin;
+            ranges[b].root_ref = kAbsentRef;
+            if (blas_root[b] != kAbsentRef) quantise = MakeQRange(begin, blas_root[b], blo, bhi, ranges[b]) && quantise;
+            for (int64_t i = 0; quantise && i < v.primitive_count; ++i) quantise = v.primitives[i].kind == 0;
         }
         layout.instances.resize(static_cast<size_t>(tl->instance_count));
         for (int32_t i = 0; i < tl->instance_count; ++i) {
@@ -668,7 +722,11 @@ yrc_status yrc_accel_create_two_level(const yrc_geometry* geometry, const yrc_tw
             dst.box_a = make_float4(box[0], box[1], box[2], box[3]);
             dst.box_b = make_float4(box[4], box[5], IntBits(valid ? blas_root[src.blas_index] : kAbsentRef),
                                     0.0f);
+            const QRange grid = valid ? ranges[src.blas_index] : QRange{};
+            dst.grid = make_float4(grid.lo[0], grid.lo[1], grid.lo[2], grid.cell);
         }
+        for (int64_t i = 0; quantise && i < tl->tlas_primitive_count; ++i) quantise = tl->tlas_primitives[i].kind != 1;
+        const int64_t tlas_begin = static_cast<int64_t>(layout.pairs.size());
         auto tlas_slot = [&](int64_t s) -> Record {
             if (s < 0 || s >= tl->tlas_primitive_index_count) return SkipRecord(kRecSkip);
             const int32_t pi = tl->tlas_primitive_indices[s];
@@ -686,7 +744,13 @@ yrc_status yrc_accel_create_two_level(const yrc_geometry* geometry, const yrc_tw
         if (!AddBvh(tl->tlas_nodes, tl->tlas_node_count, tlas_slot, layout, tlas_root, lo, hi, tlas_depth, error)) {
             return Fail(YRC_ERR_INVALID_ARGUMENT, "TLAS: " + error);
         }
+        layout.quantised_stack = QuantisedStack(tlas_depth) + QuantisedStack(blas_depth);
         tlas_depth += blas_depth;
+        QRange top{};
+        if (quantise && tlas_root != kAbsentRef && MakeQRange(tlas_begin, tlas_root, lo, hi, top)) {
+            ranges.push_back(top);
+            layout.ranges = std::move(ranges);
+        }
     } catch (const std::bad_alloc&) {
         return Fail(YRC_ERR_OUT_OF_MEMORY, "yrc_accel_create_two_level: host allocation failed");
     }
@@ -781,7 +845,8 @@ yrc_status yrc_trace_host(yrc_accel* accel, const yrc_ray* rays, int64_t count, 
         // batch that the copies of one overlap the traversal of another and
         // only one chunk's upload and readback are exposed.
         p.chunk = int64_t{1} << 19;
-        err = cudaMalloc(reinterpret_cast<void**>(&p.d_counters), sizeof(unsigned long long) * HostPipeline::kStreams);
+        err = cudaMalloc(reinterpret_cast<void**>(&p.d_counters),
+                         sizeof(unsigned long long) * (1 + kUndecidedWords) * HostPipeline::kStreams);
         for (int s = 0; s < HostPipeline::kStreams && err == cudaSuccess; ++s) {
             err = cudaStreamCreateWithFlags(&p.streams[s], cudaStreamNonBlocking);
             if (err == cudaSuccess) err = cudaMalloc(&p.d_rays[s], static_cast<size_t>(p.chunk) * sizeof(yrc_ray));
@@ -803,7 +868,10 @@ yrc_status yrc_trace_host(yrc_accel* accel, const yrc_ray* rays, int64_t count, 
     int chunk_id = 0;
     while (done < count && err == cudaSuccess) {
         const int s = chunk_id % HostPipeline::kStreams;
-        const int64_t n = std::min(p.chunk, count - done);
+        // The last chunks taper: only their traversal and readback are not
+        // hidden behind an upload.
+        const int64_t left = count - done;
+        const int64_t n = std::min({p.chunk, left, std::max<int64_t>(p.chunk / 4, (left + 1) / 2)});
         cudaStream_t st = p.streams[s];
         if (want_stats) err = cudaStreamSynchronize(st);  // host_stats buffer is reused per chunk
         if (err == cudaSuccess)
@@ -816,7 +884,7 @@ yrc_status yrc_trace_host(yrc_accel* accel, const yrc_ray* rays, int64_t count, 
                                        any ? nullptr : static_cast<yrc_hit*>(p.d_out[s]), instances ? p.d_inst[s] : nullptr,
                                        any ? static_cast<uint8_t*>(p.d_out[s]) : nullptr, want_stats ? ds : nullptr,
                                        want_stats ? ds + n : nullptr, want_stats ? ds + 2 * n : nullptr,
-                                       p.d_counters + s, st, false, accel->host_shape[any ? 1 : 0].load());
+                                       p.d_counters + s * (1 + kUndecidedWords), st, false, accel->host_shape[any ? 1 : 0].load());
         if (ls != YRC_OK) return ls;
         if (any) {
             err = cudaMemcpyAsync(occluded + done, p.d_out[s], static_cast<size_t>(n), cudaMemcpyDeviceToHost, st);

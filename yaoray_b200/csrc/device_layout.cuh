@@ -8,7 +8,7 @@
 //    fetch instead of two 32-byte fetches at unrelated addresses (left child
 //    at index+1, right child at payload_offset in RenderBvhNode).
 //      a = (L.lo.x, L.lo.y, L.lo.z, L.hi.x)   b = (L.hi.y, L.hi.z, R.lo.x, R.lo.y)
-//      c = (R.lo.z, R.hi.x, R.hi.y, R.hi.z)   d = (L.ref, R.ref, -, -)
+//      c = (R.lo.z, R.hi.x, R.hi.y, R.hi.z)   d = (L.ref, R.ref, first record of R, -)
 //    A child ref >= 0 is the child's NodePair index, kLeafBit|... (negative)
 //    is a leaf: ~first_record; kAbsentRef marks a child the reference would
 //    not test (index outside the node array).
@@ -21,8 +21,16 @@
 //    A sphere stores (center.xyz, sphere index), (radius, 0, 0, flags).
 //    In a TLAS an instance record stores (0,0,0, instance index), flags.
 //
-//  Instance (80 B, two-level only): the reference's world_to_object rows in
-//    TransformPoint order plus the BLAS root box and root ref.
+//  Instance (96 B, two-level only): the reference's world_to_object rows in
+//    TransformPoint order plus the BLAS root box, root ref and grid.
+//
+//  QNode (64 B): the up to four boxes one to three levels below a NodePair
+//    (same index), as 16-bit cells of one grid per BVH, rounded outwards
+//    (quantised.cuh). Child c = 0..3 has words 8 (c / 2) + 3 (c & 1) + axis
+//    (low half lo, high half hi) and its ref in word 8 (c / 2) + 6 + (c & 1);
+//    an absent child is the leaf of a skip record behind an empty box.
+//  Leaf boxes (32 B per record): the exact box of the leaf that starts at the
+//    record, unbounded for the others.
 #pragma once
 
 #include <cstdint>
@@ -79,6 +87,11 @@ struct alignas(16) WideNode {
 };
 static_assert(sizeof(WideNode) == 128, "WideNode must be 128 bytes");
 
+struct alignas(64) QNode {
+    uint32_t w[16];
+};
+static_assert(sizeof(QNode) == 64, "QNode must be 64 bytes");
+
 struct alignas(16) Record {
     float4 v0, v1, v2;
 };
@@ -88,8 +101,9 @@ struct alignas(16) Instance {
     float4 row0, row1, row2;  // (m[r], m[4+r], m[8+r], m[12+r]) of world_to_object
     float4 box_a;             // BLAS root lo.xyz, hi.x
     float4 box_b;             // hi.y, hi.z, root ref (int bits), BLAS root is a leaf (unused)
+    float4 grid;              // the BLAS's quantisation grid: origin, cell
 };
-static_assert(sizeof(Instance) == 80, "Instance must be 80 bytes");
+static_assert(sizeof(Instance) == 96, "Instance must be 96 bytes");
 
 // Everything a trace kernel needs, passed by value.
 struct AccelParams {
@@ -104,6 +118,10 @@ struct AccelParams {
     const WideNode* wide;      // four-wide copy of a flat triangle-only BVH, or nullptr
     int32_t wide_root;         // wide node index, ~record (leaf root) or kAbsentRef
     int32_t wide_stack_limit;  // deepest stack of the four-wide traversal
+    const QNode* qnodes;       // quantised four-wide nodes (same indices as pairs), or nullptr
+    const float4* leaf_boxes;  // two per record, with qnodes
+    float qlo[3];              // grid of the flat BVH / the TLAS
+    float qcell;
 };
 
 #if defined(__CUDACC__)
@@ -190,30 +208,37 @@ struct Nearest {
 // |det| < 1e-8 rejection, u in [0,1], v >= 0, u+v <= 1, t in (t_min, nearest.t]
 // and the equal-t tie broken toward the smaller flat_triangle_index.
 // Returns true when the candidate was accepted.
-__device__ __forceinline__ bool TriangleTest(const RayPre& r, const float4 v0, const float4 v1, const float4 v2,
-                                             float tmin, Nearest& best) {
+__device__ __forceinline__ bool TriangleIntersect(const float* o, const float* d, const float4 v0, const float4 v1,
+                                                  const float4 v2, float tmin, float tmax, float& t, float& u,
+                                                  float& v) {
     const float e1x = v1.x, e1y = v1.y, e1z = v1.z;
     const float e2x = v2.x, e2y = v2.y, e2z = v2.z;
     // pvec = Cross(d, e2)
-    const float px = __fsub_rn(__fmul_rn(r.d[1], e2z), __fmul_rn(r.d[2], e2y));
-    const float py = __fsub_rn(__fmul_rn(r.d[2], e2x), __fmul_rn(r.d[0], e2z));
-    const float pz = __fsub_rn(__fmul_rn(r.d[0], e2y), __fmul_rn(r.d[1], e2x));
+    const float px = __fsub_rn(__fmul_rn(d[1], e2z), __fmul_rn(d[2], e2y));
+    const float py = __fsub_rn(__fmul_rn(d[2], e2x), __fmul_rn(d[0], e2z));
+    const float pz = __fsub_rn(__fmul_rn(d[0], e2y), __fmul_rn(d[1], e2x));
     const float det = Dot3(e1x, e1y, e1z, px, py, pz);
     if (fabsf(det) < 1.0e-8f) return false;
     const float inv_det = __frcp_rn(det);
-    const float tx = __fsub_rn(r.o[0], v0.x);
-    const float ty = __fsub_rn(r.o[1], v0.y);
-    const float tz = __fsub_rn(r.o[2], v0.z);
-    const float u = __fmul_rn(Dot3(tx, ty, tz, px, py, pz), inv_det);
+    const float tx = __fsub_rn(o[0], v0.x);
+    const float ty = __fsub_rn(o[1], v0.y);
+    const float tz = __fsub_rn(o[2], v0.z);
+    u = __fmul_rn(Dot3(tx, ty, tz, px, py, pz), inv_det);
     if (u < 0.0f || u > 1.0f) return false;
     // qvec = Cross(tvec, e1)
     const float qx = __fsub_rn(__fmul_rn(ty, e1z), __fmul_rn(tz, e1y));
     const float qy = __fsub_rn(__fmul_rn(tz, e1x), __fmul_rn(tx, e1z));
     const float qz = __fsub_rn(__fmul_rn(tx, e1y), __fmul_rn(ty, e1x));
-    const float v = __fmul_rn(Dot3(r.d[0], r.d[1], r.d[2], qx, qy, qz), inv_det);
+    v = __fmul_rn(Dot3(d[0], d[1], d[2], qx, qy, qz), inv_det);
     if (v < 0.0f || __fadd_rn(u, v) > 1.0f) return false;
-    const float t = __fmul_rn(Dot3(e2x, e2y, e2z, qx, qy, qz), inv_det);
-    if (t <= tmin || t > best.t) return false;
+    t = __fmul_rn(Dot3(e2x, e2y, e2z, qx, qy, qz), inv_det);
+    return !(t <= tmin || t > tmax);
+}
+
+__device__ __forceinline__ bool TriangleTest(const RayPre& r, const float4 v0, const float4 v1, const float4 v2,
+                                             float tmin, Nearest& best) {
+    float t, u, v;
+    if (!TriangleIntersect(r.o, r.d, v0, v1, v2, tmin, best.t, t, u, v)) return false;
     const int32_t id = __float_as_int(v0.w);
     if (t == best.t && best.hit && best.id >= 0 && id >= best.id) return false;
     best.hit = true;

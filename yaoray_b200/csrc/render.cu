@@ -762,6 +762,7 @@ yrc_status EnsureWork(yrc_render_scene* s, int64_t capacity) {
     q.tex_normal = s->dev.texture_count > 0 ? W.Alloc<float4>(capacity) : nullptr;
     q.tex_scale = s->dev.texture_count > 0 ? W.Alloc<float4>(capacity) : nullptr;
     q.counters = W.Alloc<unsigned long long>(kCtrCount);
+    q.undecided = W.Alloc<unsigned long long>(static_cast<size_t>(kUndecidedWords));
     s->transmittance = (s->dev.any_transparent || s->dev.exact_shadows) ? W.Alloc<float4>(3 * capacity) : nullptr;
     if (s->dev.any_subsurface) {
         q.probe_ray = W.Alloc<float4>(2 * capacity);
@@ -866,6 +867,7 @@ TraceArgs ExtendTraceArgs(yrc_render_scene* s, const Queues& q) {
     ta.hits = reinterpret_cast<yrc_hit*>(q.hits);
     ta.instances = q.inst;
     ta.counter = q.counters + kCtrTrace;
+    ta.undecided = q.undecided;
     ta.error = AccelErrorWord(s->accel);
     return ta;
 }

@@ -146,6 +146,7 @@ __global__ void ResetCountersKernel(Queues q) {
         q.counters[kCtrShadow] = 0;
         q.counters[kCtrNee] = 0;
         q.counters[kCtrTrace] = 0;
+        q.undecided[0] = 0;
         q.counters[kCtrShadowTrace] = 0;
         q.counters[kCtrShadowOverflow] = 0;
         q.counters[kCtrProbe] = 0;

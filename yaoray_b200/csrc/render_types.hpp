@@ -243,6 +243,7 @@ struct Queues {
     int32_t* shadow_slot; // path * 3 + light type
     uint8_t* shadow_occluded;
     int32_t* shadow_overflow;  // shadow entries the exact loop traces (see ShadowArgs::overflow)
+    unsigned long long* undecided;  // extend rays left to the exact traversal (TraceArgs::undecided)
     int32_t* defer_paths;      // coated vertices awaiting their emissive shadow ray (kCtrDefer)
     int32_t* defer_paths2;     // ... and then their analytic / environment shadow rays (kCtrDefer2)
     int32_t* nee_paths;   // paths with pending NEE

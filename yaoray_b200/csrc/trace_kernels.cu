@@ -21,7 +21,9 @@
 //    total depth covers the BVH's longest root-to-leaf path;
 //  * nodes and leaf records are read with 128-bit read-only loads.
 #include "device_layout.cuh"
+#include "probe_loop.cuh"
 #include "render_types.hpp"
+#include "shadow_replay.cuh"
 #include "trace_kernels.hpp"
 #include "traversal.cuh"
 
@@ -232,60 +234,16 @@ __global__ void __launch_bounds__(kTraceBlock) ProbeKernel(ProbeArgs args) {
     }
 }
 
-// SampleBssrdfProbe's probe (src/integrators/bssrdf_probe.cpp:51-66) for the
-// render path: IntersectAccelerationProbe's loop (closest-hit queries with an
-// advancing cursor, target hits kept in t order, at most kProbeMaxHits)
-// run twice per probe, first to count the target hits, then to return the
-// one the selection sample picks (floor(u * count), clamped), so no per-probe
-// hit list is stored.
+// SampleBssrdfProbe's probe (ProbeLoop), one thread per probe.
 template <bool kTwo, int kTotal>
 __global__ void __launch_bounds__(kTraceBlock) RenderProbeKernel(RenderProbeArgs args) {
     __shared__ int2 s_stack[kShortStack * kTraceBlock];
     int2* col = s_stack + threadIdx.x;
     StackStore<kTotal> st;
-    Traversal s;
     const int64_t n = static_cast<int64_t>(*args.count_ptr);
     for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n;
          k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int4 target = args.targets[k];
-        const float t_min = Ld(args.rays + 2 * k).w;
-        const float t_max = Ld(args.rays + 2 * k + 1).w;
-        // pass == 0 counts; pass == 1 stops at the selected target hit
-        int32_t count = 0;
-        int32_t selected = -1;
-        float4 chosen = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (int pass = 0; pass < 2; ++pass) {
-            if (pass == 1) {
-                if (count == 0) break;
-                const float u = args.selection[2 * k].w;
-                selected = min(max(static_cast<int32_t>(u * static_cast<float>(count)), 0), count - 1);
-            }
-            int32_t seen = 0;
-            float cursor = t_min;
-            for (int iter = 0; iter < kProbeMaxIterations; ++iter) {
-                bool alive = Begin(args.accel, args.rays, k, cursor, t_max, s);
-                while (alive) alive = Step<false, false, kTwo>(args.accel, args.rays, k, s, st, col, args.error);
-                if (!s.best.hit) break;
-                const bool inst_ok = !kTwo || target.y < 0 || s.best_inst == target.y;
-                const bool is_target = (target.x >= 0 && s.best.id >= 0 && s.best.prim == target.x && inst_ok) ||
-                                       (target.z >= 0 && s.best.id == -2 - target.z);
-                if (is_target) {
-                    if (seen >= kProbeMaxHits) break;
-                    if (pass == 1 && seen == selected) {
-                        chosen = make_float4(s.best.t, __int_as_float(s.best.id), s.best.u, s.best.v);
-                        break;
-                    }
-                    ++seen;
-                }
-                float next = __fadd_rn(s.best.t, __fmul_rn(1.0e-4f, __fadd_rn(1.0f, fabsf(s.best.t))));
-                if (!(next > cursor)) next = __fadd_rn(cursor, 1.0e-4f);
-                cursor = next;
-                if (cursor >= t_max) break;
-            }
-            if (pass == 0) count = seen;
-        }
-        args.hits[k] = count;
-        args.hit[k] = chosen;
+        ProbeLoop<kTwo>(args, k, st, col);
     }
 }
 
@@ -313,7 +271,7 @@ __global__ void __launch_bounds__(kTraceBlock) RenderProbeKernel(RenderProbeArgs
 // kPooled: the launch serves the shadow queues of several jobs (ShadowPool);
 // each lane works with the job of the ray it holds.
 // kLeafBatch: leaf tests batched across the warp, as in TraceKernel.
-template <bool kTwo, int kTotal, bool kPooled = false, int kLeafBatch = 0>
+template <bool kTwo, int kTotal, bool kPooled, int kLeafBatch>
 __global__ void __launch_bounds__(kTraceBlock, kShadowBlocksPerSm)
     ShadowTransmittanceKernel(const __grid_constant__ ShadowArgs args, const __grid_constant__ ShadowPool pool) {
     __shared__ int2 s_stack[kShadowShortStack * kTraceBlock];
@@ -336,111 +294,6 @@ __global__ void __launch_bounds__(kTraceBlock, kShadowBlocksPerSm)
     bool alive = false;
     bool exhausted = false;
 
-    // The reference loop over the kept clear surfaces; returns the RGB
-    // transmittance, w = 1 when visible, all 0 when occluded.
-    auto replay = [&]() -> float4 {
-        const float4 ra = Ld(A->rays + 2 * ray);
-        const float4 rb = Ld(A->rays + 2 * ray + 1);
-        float o[3] = {ra.x, ra.y, ra.z};
-        const float d[3] = {rb.x, rb.y, rb.z};
-        float remaining = rb.w;
-        float T[3] = {1.0f, 1.0f, 1.0f}, mc[3] = {1.0f, 1.0f, 1.0f}, md = 1.0f;
-        bool medium = false;
-        float qmin = ra.w;   // t_min of the current query
-        float off = 0.0f;    // distance from the ray origin to the current query's origin
-        const float4 occluded = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        auto black = [&]() { return fmaxf(T[0], fmaxf(T[1], T[2])) <= 1.0e-6f; };
-        auto beer = [&](float dist) {
-            if (dist <= 0.0f || md <= 0.0f) return;
-            const float inv = 1.0f / md;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float c = fminf(fmaxf(mc[k], 1.0e-6f), 1.0f);
-                T[k] = T[k] * expf(logf(c) * dist * inv);
-            }
-        };
-        int k = 0;
-        for (int query = 0; query < kClearHits; ++query) {
-            const bool finite = isfinite(remaining);
-            float t = 0.0f;
-            int32_t id = 0;
-            bool found = false;
-            for (; k < clear.n; ++k) {
-                t = __fsub_rn(clear.t[k * kTraceBlock], off);
-                if (t > qmin && t <= remaining) {
-                    id = clear.id[k * kTraceBlock];
-                    found = true;
-                    ++k;
-                    break;
-                }
-            }
-            if (!found) {
-                // A surface beyond the kept ones would be this query's
-                // answer: the exact loop traces this ray instead.
-                if (clear.dropped) return make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-                if (medium) {
-                    if (!finite) return occluded;
-                    beer(remaining);
-                }
-                return black() ? occluded : make_float4(T[0], T[1], T[2], 1.0f);
-            }
-            if (medium) {
-                beer(t);
-                if (black()) return occluded;
-            }
-            const int32_t material = id >= 0 ? A->prim_material[A->tri_prim[id]] : A->sphere_material[-2 - id];
-            if (material < 0 || (A->materials[material].kind != 2 && A->materials[material].kind != 3)) {
-                return occluded;
-            }
-            const DevMaterial& m = A->materials[material];
-            float hp[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) hp[c] = __fadd_rn(o[c], __fmul_rn(d[c], t));
-            if (m.kind == 3) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) T[c] = T[c] * fminf(fmaxf(m.reflectance[c], 0.0f), 1.0f);
-                if (black()) return occluded;
-            } else if (medium) {
-                medium = false;
-                mc[0] = mc[1] = mc[2] = 1.0f;
-                md = 1.0f;
-            } else {
-                medium = true;
-                mc[0] = m.absorption_color[0];
-                mc[1] = m.absorption_color[1];
-                mc[2] = m.absorption_color[2];
-                md = m.absorption_distance;
-            }
-            const float bias = fmaxf(1.0e-4f, fmaxf(fabsf(hp[0]), fmaxf(fabsf(hp[1]), fabsf(hp[2]))) * 1.0e-5f);
-            if (finite) {
-                remaining = __fsub_rn(remaining, __fadd_rn(t, bias));
-                if (remaining <= 0.0f) return black() ? occluded : make_float4(T[0], T[1], T[2], 1.0f);
-            }
-#pragma unroll
-            for (int c = 0; c < 3; ++c) o[c] = __fadd_rn(hp[c], __fmul_rn(d[c], bias));
-            off = __fadd_rn(off, __fadd_rn(t, bias));
-            qmin = 1.0e-5f;
-        }
-        return occluded;  // the reference gives up after 16 queries
-    };
-    auto finish = [&]() {
-        const int32_t slot = A->out_index[ray];
-        float4 tr;
-        if (s.best.hit) {
-            tr = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        } else if (!s.saw) {
-            tr = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-        } else {
-            tr = replay();
-            if (tr.w < 0.0f) {
-                const unsigned long long o = atomicAdd(A->overflow_count, 1ull);
-                A->overflow[o] = static_cast<int32_t>(ray);
-                return;
-            }
-        }
-        A->transmittance[slot] = tr;
-        if (tr.w == 0.0f) CountLanes(A->occluded_count);
-    };
     for (;;) {
         const unsigned need = __ballot_sync(kFull, !alive && !exhausted);
         if (need) {
@@ -467,7 +320,7 @@ __global__ void __launch_bounds__(kTraceBlock, kShadowBlocksPerSm)
                     clear.n = 0;
                     clear.dropped = false;
                     alive = Begin(acc, A->rays, ray, tmin, b.w, s);
-                    if (!alive) finish();
+                    if (!alive) FinishShadow(*A, ray, s.best.hit, s.saw, clear);
                 }
             }
         }
@@ -475,40 +328,19 @@ __global__ void __launch_bounds__(kTraceBlock, kShadowBlocksPerSm)
             if (__all_sync(kFull, exhausted)) break;
             continue;
         }
-        if constexpr (kLeafBatch > 0) {
 #pragma unroll 1
-            for (int k = 0; k < 8; ++k) {
-                const unsigned at_leaf = __ballot_sync(kFull, alive && s.cur < 0);
-                const unsigned at_node = __ballot_sync(kFull, alive && s.cur >= 0);
-                if (!(at_leaf | at_node)) break;
-                const bool leaves = at_node == 0u || __popc(at_leaf) >= kLeafBatch;
-                if (alive && (s.cur >= 0 || leaves)) {
-                    alive = Step<true, false, kTwo, StackStore<kTotal, kTraceBlock, kShadowShortStack>, true>(
-                        acc, A->rays, ray, s, st, col, A->error, A->tri_clear, A->sphere_clear, &clear);
-                    if (!alive) finish();
-                }
-            }
-        } else {
-#pragma unroll 1
-            for (int k = 0; k < 8 && alive; ++k) {
+        for (int k = 0; k < 8; ++k) {
+            const unsigned at_leaf = __ballot_sync(kFull, alive && s.cur < 0);
+            const unsigned at_node = __ballot_sync(kFull, alive && s.cur >= 0);
+            if (!(at_leaf | at_node)) break;
+            const bool leaves = at_node == 0u || __popc(at_leaf) >= kLeafBatch;
+            if (alive && (s.cur >= 0 || leaves)) {
                 alive = Step<true, false, kTwo, StackStore<kTotal, kTraceBlock, kShadowShortStack>, true>(
                     acc, A->rays, ray, s, st, col, A->error, A->tri_clear, A->sphere_clear, &clear);
-                if (!alive) finish();
+                if (!alive) FinishShadow(*A, ray, s.best.hit, s.saw, clear);
             }
         }
     }
-}
-
-template <typename Kernel>
-cudaError_t PersistentGrid(Kernel kernel, int block, int64_t count, int sm_count, int64_t& blocks) {
-    int per_sm = 0;
-    const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
-    if (err != cudaSuccess) return err;
-    if (per_sm < 1) per_sm = 1;
-    blocks = static_cast<int64_t>(per_sm) * sm_count;
-    const int64_t needed = (count + block - 1) / block;
-    if (blocks > needed) blocks = needed < 1 ? 1 : needed;
-    return cudaSuccess;
 }
 
 template <bool kAny, bool kStats, bool kTwo, int kTotal, int kBlock, int kStepsPerRefill, int kMinBlocks,
@@ -522,29 +354,25 @@ cudaError_t LaunchOne(const TraceArgs& args, cudaStream_t stream, int sm_count) 
     return cudaGetLastError();
 }
 
-// The tunable launch shapes (block size, node visits between ray refills,
-// minimum resident blocks for the register budget). Index 0 is the default;
-// the autotuner times the rest on the actual accelerator.
+// The launch shapes over the exact nodes: leaf batch 16 at 64 registers (9, 12),
+// leaf batch 8 at 56 (10, 15, 16), else leaf batch 8 unbounded. What shape 0
+// and the shapes 1-6 stood for, leaves run as soon as one lane is at one, was
+// slower everywhere: 2M triangles, 8M incoherent rays 2.99 ms against 2.30
+// (shape 8) and 2.23 (15), camera rays 0.49 against 0.42 and 0.40, two-level
+// 1.19 against 0.84 (8) and 0.70 (12), any hit 0.96 against 0.60 (12).
 template <bool kAny, bool kStats, bool kTwo, int kTotal, bool kWide = false>
 cudaError_t LaunchShape(const TraceArgs& args, int shape, cudaStream_t stream, int sm_count) {
-    switch (kStats ? 0 : shape) {
-        case 1: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 4, 1, kWide>(args, stream, sm_count);
-        case 2: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 16, 1, kWide>(args, stream, sm_count);
-        case 3: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 12, kWide>(args, stream, sm_count);
-        case 4: return LaunchOne<kAny, kStats, kTwo, kTotal, 64, 8, 1, kWide>(args, stream, sm_count);
-        case 5: return LaunchOne<kAny, kStats, kTwo, kTotal, 256, 8, 1, kWide>(args, stream, sm_count);
-        case 6: return LaunchOne<kAny, kStats, kTwo, kTotal, 64, 8, 24, kWide>(args, stream, sm_count);
-        case 7: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 1, kWide, 4>(args, stream, sm_count);
-        case 8: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 1, kWide, 8>(args, stream, sm_count);
-        case 9: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 1, kWide, 16>(args, stream, sm_count);
-        case 10: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 12, kWide, 8>(args, stream, sm_count);
-        case 11: return LaunchOne<kAny, kStats, kTwo, kTotal, 256, 8, 1, kWide, 8>(args, stream, sm_count);
-        case 12: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 8, kWide, 16>(args, stream, sm_count);
-        case 13: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 16, 1, kWide, 8>(args, stream, sm_count);
-        case 14: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 32, 1, kWide, 8>(args, stream, sm_count);
-        case 15: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 9, kWide, 8>(args, stream, sm_count);
-        case 16: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 10, kWide, 8>(args, stream, sm_count);
-        default: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 1, kWide>(args, stream, sm_count);
+    if constexpr (kStats) {
+        return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 1, kWide>(args, stream, sm_count);
+    } else {
+        switch (shape) {
+            case 9:
+            case 12: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 8, kWide, 16>(args, stream, sm_count);
+            case 10:
+            case 15:
+            case 16: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 9, kWide, 8>(args, stream, sm_count);
+            default: return LaunchOne<kAny, kStats, kTwo, kTotal, 128, 8, 1, kWide, 8>(args, stream, sm_count);
+        }
     }
 }
 
@@ -560,7 +388,7 @@ cudaError_t LaunchWide(const TraceArgs& args, int shape, cudaStream_t stream, in
     if (args.accel.wide_stack_limit <= 64) {
         return LaunchShape<kAny, false, false, 64, true>(args, shape, stream, sm_count);
     }
-    return LaunchOne<kAny, false, false, kMaxTraceStack, 128, 8, 1, true>(args, stream, sm_count);
+    return LaunchOne<kAny, false, false, kMaxTraceStack, 128, 8, 1, true, 8>(args, stream, sm_count);
 }
 
 template <bool kTwo, int kTotal>
@@ -576,11 +404,10 @@ cudaError_t LaunchProbeOne(const ProbeArgs& args, cudaStream_t stream, int sm_co
 template <bool kTwo, int kTotal, bool kPooled = false>
 cudaError_t LaunchShadowOne(const ShadowArgs& args, const ShadowPool& pool, cudaStream_t stream, int sm_count) {
     // A pooled launch batches leaf tests by 8; a single one as its shape asks
-    // (leaf batch 4 runs as 8).
+    // (16, else 8).
     auto kernel = kPooled                  ? ShadowTransmittanceKernel<kTwo, kTotal, kPooled, 8>
                   : args.leaf_batch >= 16 ? ShadowTransmittanceKernel<kTwo, kTotal, kPooled, 16>
-                  : args.leaf_batch > 0   ? ShadowTransmittanceKernel<kTwo, kTotal, kPooled, 8>
-                                          : ShadowTransmittanceKernel<kTwo, kTotal, kPooled, 0>;
+                                          : ShadowTransmittanceKernel<kTwo, kTotal, kPooled, 8>;
     int64_t blocks = 0;
     const cudaError_t err =
         PersistentGrid(kernel, kTraceBlock, kPooled ? pool.capacity : args.capacity, sm_count, blocks);
@@ -613,6 +440,7 @@ cudaError_t LaunchRenderProbeOne(const RenderProbeArgs& args, cudaStream_t strea
 }
 
 cudaError_t LaunchRenderProbe(const RenderProbeArgs& args, cudaStream_t stream, int sm_count) {
+    if (args.accel.qnodes) return LaunchQRenderProbe(args, stream, sm_count);
     const bool two = args.accel.two_level != 0;
     const bool deep = args.accel.stack_limit > 64;
     if (two) return deep ? LaunchRenderProbeOne<true, kMaxTraceStack>(args, stream, sm_count)
@@ -622,6 +450,7 @@ cudaError_t LaunchRenderProbe(const RenderProbeArgs& args, cudaStream_t stream, 
 }
 
 cudaError_t LaunchShadowTransmittance(const ShadowArgs& args, cudaStream_t stream, int sm_count) {
+    if (args.accel.qnodes) return LaunchQShadow(args, stream, sm_count);
     const bool two = args.accel.two_level != 0;
     const bool deep = args.accel.stack_limit > 64;
     const ShadowPool none{};
@@ -663,6 +492,12 @@ cudaError_t LaunchTrace(const TraceArgs& args, bool any_hit, bool stats, int sha
     const bool two = args.accel.two_level != 0;
     if (!two && !stats && args.accel.wide) {
         return any_hit ? LaunchWide<true>(args, shape, stream, sm_count) : LaunchWide<false>(args, shape, stream, sm_count);
+    }
+    // Closest hits over the quantised nodes take a second launch (RetraceKernel,
+    // 2-3 us): too much for the smallest calls (a thousand rays, 12K triangles:
+    // 23.5 us a call against 21).
+    if (!stats && args.accel.qnodes && (any_hit || args.count >= kQuantisedMinRays)) {
+        return LaunchQTrace(args, any_hit, shape, stream, sm_count);
     }
     if (any_hit) {
         if (two) return stats ? LaunchDepth<true, true, true>(args, shape, stream, sm_count)

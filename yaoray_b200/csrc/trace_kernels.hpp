@@ -13,6 +13,14 @@ namespace yrc {
 constexpr int kTraceBlock = 128;    // threads per block
 constexpr int kShortStack = 12;     // stack entries per thread kept in shared memory
 constexpr int kTraceShapes = 17;     // launch shapes the autotuner may choose from
+constexpr int kQuantisedStack = 96;  // stack entries of the quantised traversal; deeper BVHs take the exact nodes
+constexpr int kQuantisedExactStack = 64;  // exact stack entries for what it leaves to the exact nodes
+// Rays a quantised closest-hit launch may list for the exact traversal (their
+// count, then the list); beyond these it scans the hits for the mark.
+constexpr int kUndecidedMax = 16382;
+constexpr int64_t kUndecidedWords = 1 + kUndecidedMax / 2;  // 64-bit words, the count included
+constexpr int64_t kQuantisedMinRays = int64_t{1} << 15;
+constexpr int32_t kUndecidedId = INT32_MIN;
 constexpr int kMaxTraceStack = 256; // deepest traversal stack any kernel supports
 
 // Status bits a kernel may set in the accelerator's device error word.
@@ -29,6 +37,7 @@ struct TraceArgs {
     uint32_t* triangle_tests;
     uint32_t* sphere_tests;
     unsigned long long* counter;  // ray work counter, zeroed before the launch
+    unsigned long long* undecided;  // closest hits over quantised nodes: kUndecidedWords, the first zeroed before the launch
     int* error;                   // device error word
     const unsigned long long* count_ptr;  // optional: ray count read on the device (count = capacity)
     const int32_t* out_index;             // optional: any-hit output slot per ray
@@ -138,6 +147,10 @@ cudaError_t LaunchShadowTransmittance(const ShadowArgs& args, cudaStream_t strea
 
 cudaError_t LaunchTrace(const TraceArgs& args, bool any_hit, bool stats, int shape, cudaStream_t stream,
                         int sm_count);
+// LaunchTrace over the quantised nodes (qtrace_kernels.cu); accel.qnodes set.
+cudaError_t LaunchQTrace(const TraceArgs& args, bool any_hit, int shape, cudaStream_t stream, int sm_count);
+cudaError_t LaunchQShadow(const ShadowArgs& args, cudaStream_t stream, int sm_count);
+cudaError_t LaunchQRenderProbe(const RenderProbeArgs& args, cudaStream_t stream, int sm_count);
 cudaError_t LaunchProbe(const ProbeArgs& args, cudaStream_t stream, int sm_count);
 
 // Ray reordering ahead of a traversal launch (ray_order.cu).

@@ -466,5 +466,19 @@ __device__ __forceinline__ bool Step(const AccelParams& a, const float4* rays, i
     return Pop<kAny, kTwo>(rays, ray, s, st, col);
 }
 
+// Blocks of a persistent launch: what the device holds at once, or fewer
+// where `count` rays fill fewer.
+template <typename Kernel>
+cudaError_t PersistentGrid(Kernel kernel, int block, int64_t count, int sm_count, int64_t& blocks) {
+    int per_sm = 0;
+    const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
+    if (err != cudaSuccess) return err;
+    if (per_sm < 1) per_sm = 1;
+    blocks = static_cast<int64_t>(per_sm) * sm_count;
+    const int64_t needed = (count + block - 1) / block;
+    if (blocks > needed) blocks = needed < 1 ? 1 : needed;
+    return cudaSuccess;
+}
+
 }  // namespace
 }  // namespace yrc
